@@ -757,8 +757,12 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const DecodeParams p)
     const int hk = head / p.group, steps = steps_of(p, b);
     const int first = (entry_begin + hk * steps) / shares.share;
     parts = (entry_begin + hk * steps + steps - 1) / shares.share - first + 1;
-    if (parts == 1)
-      return; // that block has written the result
+    if (parts == 1) { // that block has written the result
+      // Waited for all the same: launched early, this grid may finish only after the split kernel has, because whatever
+      // comes next depends on this grid alone.  Where no row has two parts (every entry within one share) no other block waits.
+      pdl_wait();
+      return;
+    }
     part0 = ((int64_t)first + (int64_t)b * p.h_k + hk) * p.rows_per_kv + i * p.group + head % p.group;
     part_step = p.rows_per_kv;
   }
