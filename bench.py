@@ -893,8 +893,8 @@ class AttnFwd(Workload):
 class AttnFwdBwd(AttnFwd):
     """FlashAttn fwd+bwd: bf16 Q,K,V,dO [B=8, S=4096, H=32, D=128] N(0,1), causal, scale 1/sqrt(128)"""
     key, name = "attn_fwd_bwd", "flash_attn_fwd_bwd_bf16_b8_s4096_h32_d128_causal"
-    kernel = "flash_fwd_kernel, bwd_dot_do_o_kernel, flash_bwd_kernel<dK/dV>, flash_bwd_kernel<dQ> (whole step)"
-    launches = 4
+    kernel = "flash_fwd_kernel, bwd_dot_do_o_kernel, flash_bwd_kernel (whole step)"
+    launches = 3
     with_bwd = True
 
 

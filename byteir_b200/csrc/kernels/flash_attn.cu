@@ -755,25 +755,26 @@ int make_qkv_map(CUtensorMap *map, bool bf16, const void *base, int64_t d, int64
 // =============================================================================
 // backward
 // =============================================================================
-// Three kernels, no atomics, so the result is a function of the inputs alone
+// Two kernels, no atomics, so the result is a function of the inputs alone
 // (the reference adds dQ partials with atomicAdd, flash_bwd_kernel.h:663):
 //   1. bwd_dot_do_o_kernel   D[b,h,i] = sum_d dO * O  (f32)
-//   2. bwd_dkdv_kernel       one block per 128 keys; walks over the query tiles
-//                            that see them; dK, dV accumulate in tensor memory
-//   3. bwd_dq_kernel         one block per 128 queries; walks over the key tiles;
-//                            dQ accumulates in tensor memory
-// Kernels 2 and 3 both recompute P = exp2(S * scale * log2e - LSE * log2e) and
+//   2. flash_bwd_kernel      two passes in one grid:
+//      dK/dV   one block per 128 keys; walks over the query tiles that see them;
+//              dK, dV accumulate in tensor memory
+//      dQ      one block per 128 queries; walks over the key tiles; dQ accumulates
+//              in tensor memory
+// Both passes recompute P = exp2(S * scale * log2e - LSE * log2e) and
 // dS = P o (dP - D) from the saved LSE, as the reference does
 // (flash_bwd_kernel.h:472-580); P and dS are rounded to the storage type before
-// the following products.  Kernel 2 works on transposed tiles (S^T = K Q^T), so
+// the following products.  The dK/dV pass works on transposed tiles (S^T = K Q^T), so
 // that the thread that owns a key row writes rows of P^T and dS^T, which are the
 // K-major A operands of dV += P^T dO and dK += dS^T Q.
 
 // Tensor-memory columns.  S / dP tiles are 128 x 64 (64 streamed rows per step) and
 // double-buffered, one buffer per elementwise group; P and dS (16 bit) overwrite the
 // front of the S / dP buffer they were computed from.
-//   dK/dV kernel: S^T 0,64 | dP^T 128,192 | dV 256 | dK 384
-//   dQ kernel:    Q 0 | dO 64 (A operands) | S 128,192 | dP 256,320 | dQ 384
+//   dK/dV pass: S^T 0,64 | dP^T 128,192 | dV 256 | dK 384
+//   dQ pass:    Q 0 | dO 64 (A operands) | S 128,192 | dP 256,320 | dQ 384
 constexpr int kBwdBN = 64;       // streamed rows per step
 constexpr int kBwdStages = 4;    // ring depth of the streamed (row tile, row tile) pairs
 constexpr uint32_t kStrTileBytes = kBwdBN * kD * 2; // 16 KiB: [2 column blocks][64 rows][128 B]
@@ -788,19 +789,35 @@ struct BwdParams {
   uint32_t wait_polls;
   int debug_skip_arrive;
   int d; // head dim, <= 128
-  bool tiles_last; // grid (heads, batch, tiles) instead of (tiles, heads, batch)
+};
+
+// The blocks of one pass, in the order in which they start: tile by tile of one (batch, head) after the other, or
+// (tiles_last) the first tile of every (batch, head), then the second ...
+struct BwdPass {
+  uint32_t tiles, heads, batch;
+  bool tiles_last;
+  __device__ __forceinline__ void at(uint32_t i, int &tile, int &head, int &b) const {
+    const uint32_t inner = tiles_last ? heads : tiles, middle = tiles_last ? batch : heads;
+    const uint32_t rest = i / inner, x = i - rest * inner, z = rest / middle, y = rest - z * middle;
+    tile = tiles_last ? z : x, head = tiles_last ? x : y, b = tiles_last ? y : z;
+  }
+};
+struct BwdMaps {
+  CUtensorMap q, k, v, dout;         // boxes of 128 rows: the tiles that a block owns
+  CUtensorMap q64, k64, v64, dout64; // boxes of 64 rows: the tiles that it streams
+  CUtensorMap dq, dk, dv;
 };
 
 struct BwdShared {
   uint64_t bar_resident;                          // the block's own tiles (K,V or Q,dO) in shared memory
-  uint64_t res_ready;                             // ... and, dQ kernel, copied to tensor memory
+  uint64_t res_ready;                             // ... and, dQ pass, copied to tensor memory
   uint64_t full[kBwdStages], empty[kBwdStages];   // streamed tile pairs
   uint64_t sdp_full[2];                           // S / dP of a group's tile are in tensor memory
   uint64_t pds_full[2];                           // the group has written P / dS
   uint64_t all_done;                              // every MMA of the block has completed
   uint32_t tmem_base;
   int failed;
-  // dK/dV kernel: -lse * log2e and -dsum of the streamed queries [group][parity][row], negated
+  // dK/dV pass: -lse * log2e and -dsum of the streamed queries [group][parity][row], negated
   // so that pairs of them are addends of packed FMAs / ADDs (read four at a time: 16-byte aligned)
   alignas(16) float neg_lse2[2][2][kBwdBN];
   alignas(16) float neg_dsum[2][2][kBwdBN];
@@ -893,16 +910,12 @@ __global__ void __launch_bounds__(256)
 // 4..7 and 8..11 two elementwise groups that take the streamed tiles alternately, so that the
 // tensor core works on one group's products while the other group computes P and dS.
 // P^T / dS^T (dS) go back to tensor memory and are the A operands of the accumulating
-// products; in the dQ kernel Q and dO are A operands from tensor memory as well.
+// products; in the dQ pass Q and dO are A operands from tensor memory as well.
 template <bool kBF16, bool kDKDV, bool kNarrow>
-__global__ void __launch_bounds__(kThreads, 1)
-    flash_bwd_kernel(const __grid_constant__ CUtensorMap res0_map, // K (kDKDV) or Q, 128-row boxes
-                     const __grid_constant__ CUtensorMap res1_map, // V (kDKDV) or dO
-                     const __grid_constant__ CUtensorMap str0_map, // Q (kDKDV) or K, 64-row boxes
-                     const __grid_constant__ CUtensorMap str1_map, // dO (kDKDV) or V
-                     const __grid_constant__ CUtensorMap out0_map, // dK (kDKDV) or dQ
-                     const __grid_constant__ CUtensorMap out1_map, // dV (kDKDV), unused otherwise
-                     const BwdParams p) {
+__device__ __forceinline__ void bwd_block(const BwdMaps &m, const BwdParams &p, const BwdPass &pass, uint32_t block) {
+  const CUtensorMap &res0_map = kDKDV ? m.k : m.q, &res1_map = kDKDV ? m.v : m.dout;
+  const CUtensorMap &str0_map = kDKDV ? m.q64 : m.k64, &str1_map = kDKDV ? m.dout64 : m.v64;
+  const CUtensorMap &out0_map = kDKDV ? m.dk : m.dq, &out1_map = m.dv; // the latter kDKDV only
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem =
       reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -911,16 +924,15 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned char *sStr = sRes1 + kTileBytes;        // [stage][2 tiles of 64 rows]
   BwdShared *ss = reinterpret_cast<BwdShared *>(sStr + kBwdStages * 2 * kStrTileBytes);
 
-  constexpr uint32_t kColA0 = 0, kColA1 = 64;                    // dQ kernel: Q, dO
+  constexpr uint32_t kColA0 = 0, kColA1 = 64;                    // dQ pass: Q, dO
   constexpr uint32_t kColS = kDKDV ? 0 : 128;                    // + 64 * group
   constexpr uint32_t kColDP = kDKDV ? 128 : 256;                 // + 64 * group
   constexpr uint32_t kColAcc0 = kDKDV ? 256 : 384, kColAcc1 = 384; // dV | dK, or dQ
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31; // warp: known uniform
   const HeadSteps<kNarrow> hd(p.d);
-  // blocks start in the order of their linear index, the longest tile first either way (own_tile below)
-  const int tile_rank = p.tiles_last ? blockIdx.z : blockIdx.x;
-  const int b = p.tiles_last ? blockIdx.y : blockIdx.z;
+  int tile_rank, head, b; // blocks start in the order of their index, the longest tile first (own_tile below)
+  pass.at(block, tile_rank, head, b);
   const int64_t shift = p.Sk - p.Sq;
   const bool right_bounded = p.window_right >= 0;
   const bool left_bounded = p.window_left >= 0;
@@ -928,10 +940,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int n_q_tiles = (int)((p.Sq + kBM - 1) / kBM);
 
   // the tile this block owns, and the range of streamed 64-row tiles [t_begin, t_end)
-  int own_tile, head, t_begin, t_end, heads_in_loop;
-  if (kDKDV) {
+  int own_tile, t_begin, t_end, heads_in_loop;
+  if (kDKDV) { // `head` is a key/value head
     own_tile = tile_rank;
-    head = p.tiles_last ? blockIdx.x : blockIdx.y; // key/value head
     heads_in_loop = group;
     t_begin = 0;
     t_end = (int)((p.Sq + kBwdBN - 1) / kBwdBN);
@@ -945,7 +956,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     own_tile = n_q_tiles - 1 - tile_rank;
-    head = p.tiles_last ? blockIdx.x : blockIdx.y; // query head
     heads_in_loop = 1;
     t_begin = 0;
     t_end = (int)((p.Sk + kBwdBN - 1) / kBwdBN);
@@ -985,15 +995,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = ss->tmem_base;
-  // The three kernels of a backward are a chain of dependent launches.  The dK/dV pass waits for the row sums (kernel 1)
-  // and only then lets the dQ pass start: whatever dQ blocks find a free SM while the last dK/dV blocks run may begin at
-  // once, because they need kernel 1 alone.  The dQ pass waits at its end, so that it is never complete before the
-  // dK/dV pass is.  bf16 causal, forward and backward: [2, 300, 8, 128] 39 -> 24 us, [2, 1024, 16 / 8, 128] 92 -> 72,
-  // [1, 2048, 32 / 4, 128] 363 -> 332.
-  if (kDKDV) {
-    pdl_wait();
-    pdl_launch_dependents();
-  }
+  pdl_wait(); // the row sums, and everything in front of them; the set-up above overlaps their end
 
   // streamed iteration -> (query head, streamed tile index)
   auto iter_head = [&](int it) { return kDKDV ? head * group + it / tiles_per_head : head; };
@@ -1313,25 +1315,38 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   if (threadIdx.x == 0 && ss->failed)
     g_attn_status = 3; // dq / dk / dv of this block were not stored
-  if (!kDKDV)
-    pdl_wait();
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem, kTmemCols);
   }
 }
 
-template <bool kBF16, bool kDKDV, bool kNarrow>
-int launch_bwd(const CUtensorMap &res0, const CUtensorMap &res1, const CUtensorMap &str0, const CUtensorMap &str1,
-               const CUtensorMap &out0, const CUtensorMap &out1, const BwdParams &p, dim3 grid,
-               cudaStream_t stream) {
+// Both passes are one grid, the dK/dV blocks in front: neither reads what the other writes, and the dQ blocks start on the
+// SMs that the last dK/dV blocks leave.  Every block waits for the row sums by itself.  (As two dependent launches the dQ blocks
+// that start early have to read the row sums without a wait of their own.  60 drawn shapes: one grid 2 % faster, the same bits;
+// bf16 [8, 4096, 32, 128] causal, forward and backward, 5.36 ms either way.)
+template <bool kBF16, bool kNarrow>
+__global__ void __launch_bounds__(kThreads, 1)
+    flash_bwd_kernel(const __grid_constant__ BwdMaps m, const __grid_constant__ BwdParams p, const BwdPass kv, const BwdPass q,
+                     uint32_t kv_blocks) {
+  if (blockIdx.x < kv_blocks)
+    bwd_block<kBF16, true, kNarrow>(m, p, kv, blockIdx.x);
+  else
+    bwd_block<kBF16, false, kNarrow>(m, p, q, blockIdx.x - kv_blocks);
+}
+
+template <bool kBF16, bool kNarrow>
+int launch_bwd(const BwdMaps &m, const BwdParams &p, const BwdPass &kv, const BwdPass &q, cudaStream_t stream) {
+  const int64_t kv_blocks = (int64_t)kv.tiles * kv.heads * kv.batch, q_blocks = (int64_t)q.tiles * q.heads * q.batch;
+  if (kv_blocks + q_blocks > 0x7fffffffLL)
+    return B200_ERR_UNSUPPORTED;
   const size_t smem = (size_t)2 * kTileBytes + (size_t)kBwdStages * 2 * kStrTileBytes + sizeof(BwdShared) + 1024;
   // the attribute belongs to the current device's context: set on every call (a host-side table write)
-  if (int rc = check_cuda(cudaFuncSetAttribute(flash_bwd_kernel<kBF16, kDKDV, kNarrow>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
+  if (int rc = check_cuda(cudaFuncSetAttribute(flash_bwd_kernel<kBF16, kNarrow>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem)))
     return rc;
-  return launch_pdl(flash_bwd_kernel<kBF16, kDKDV, kNarrow>, grid, dim3(kThreads), smem, stream, res0, res1, str0, str1,
-                    out0, out1, p);
+  return launch_pdl(flash_bwd_kernel<kBF16, kNarrow>, dim3((unsigned)(kv_blocks + q_blocks)), dim3(kThreads), smem, stream, m, p, kv,
+                    q, (uint32_t)kv_blocks);
 }
 
 } // namespace
@@ -1451,23 +1466,23 @@ extern "C" int b200_flash_attn_bwd(int dtype, const void *dout, const void *q, c
   // dq / dk / dv use the strides of q / k / v and dout those of out, as in the
   // reference's custom call (flash_api.cu:370-381)
   // q / k / v / dout are read both as a block's own 128-row tile and as streamed 64-row tiles
-  CUtensorMap q_map, k_map, v_map, do_map, q64_map, k64_map, v64_map, do64_map, dq_map, dk_map, dv_map;
+  BwdMaps bm;
   struct {
     CUtensorMap *m;
     const void *base;
     int64_t heads, seq, hs, rs, bs;
     uint32_t box_rows;
-  } maps[] = {{&q_map, q, a.h, a.seqlen_q, a.q_head_stride, a.q_row_stride, a.q_batch_stride, 128},
-              {&k_map, k, a.h_k, a.seqlen_k, a.k_head_stride, a.k_row_stride, a.k_batch_stride, 128},
-              {&v_map, v, a.h_k, a.seqlen_k, a.v_head_stride, a.v_row_stride, a.v_batch_stride, 128},
-              {&do_map, dout, a.h, a.seqlen_q, a.o_head_stride, a.o_row_stride, a.o_batch_stride, 128},
-              {&q64_map, q, a.h, a.seqlen_q, a.q_head_stride, a.q_row_stride, a.q_batch_stride, kBwdBN},
-              {&k64_map, k, a.h_k, a.seqlen_k, a.k_head_stride, a.k_row_stride, a.k_batch_stride, kBwdBN},
-              {&v64_map, v, a.h_k, a.seqlen_k, a.v_head_stride, a.v_row_stride, a.v_batch_stride, kBwdBN},
-              {&do64_map, dout, a.h, a.seqlen_q, a.o_head_stride, a.o_row_stride, a.o_batch_stride, kBwdBN},
-              {&dq_map, dq, a.h, a.seqlen_q, a.q_head_stride, a.q_row_stride, a.q_batch_stride, 128},
-              {&dk_map, dk, a.h_k, a.seqlen_k, a.k_head_stride, a.k_row_stride, a.k_batch_stride, 128},
-              {&dv_map, dv, a.h_k, a.seqlen_k, a.v_head_stride, a.v_row_stride, a.v_batch_stride, 128}};
+  } maps[] = {{&bm.q, q, a.h, a.seqlen_q, a.q_head_stride, a.q_row_stride, a.q_batch_stride, 128},
+              {&bm.k, k, a.h_k, a.seqlen_k, a.k_head_stride, a.k_row_stride, a.k_batch_stride, 128},
+              {&bm.v, v, a.h_k, a.seqlen_k, a.v_head_stride, a.v_row_stride, a.v_batch_stride, 128},
+              {&bm.dout, dout, a.h, a.seqlen_q, a.o_head_stride, a.o_row_stride, a.o_batch_stride, 128},
+              {&bm.q64, q, a.h, a.seqlen_q, a.q_head_stride, a.q_row_stride, a.q_batch_stride, kBwdBN},
+              {&bm.k64, k, a.h_k, a.seqlen_k, a.k_head_stride, a.k_row_stride, a.k_batch_stride, kBwdBN},
+              {&bm.v64, v, a.h_k, a.seqlen_k, a.v_head_stride, a.v_row_stride, a.v_batch_stride, kBwdBN},
+              {&bm.dout64, dout, a.h, a.seqlen_q, a.o_head_stride, a.o_row_stride, a.o_batch_stride, kBwdBN},
+              {&bm.dq, dq, a.h, a.seqlen_q, a.q_head_stride, a.q_row_stride, a.q_batch_stride, 128},
+              {&bm.dk, dk, a.h_k, a.seqlen_k, a.k_head_stride, a.k_row_stride, a.k_batch_stride, 128},
+              {&bm.dv, dv, a.h_k, a.seqlen_k, a.v_head_stride, a.v_row_stride, a.v_batch_stride, 128}};
   for (auto &m : maps)
     if (int rc = make_qkv_map(m.m, bf16, m.base, a.d, m.heads, m.seq, a.b, m.hs, m.rs, m.bs, m.box_rows))
       return rc;
@@ -1494,23 +1509,11 @@ extern "C" int b200_flash_attn_bwd(int dtype, const void *dout, const void *q, c
   p.debug_skip_arrive = g_debug_skip_arrive;
   p.d = (int)a.d;
   // what the dK/dV pass streams is Q and dO, the dQ pass K and V
-  BwdParams p_kv = p, p_q = p;
-  constexpr int64_t kMostRows = 65535 * 128; // as many tiles as fit grid dimension z
-  p_kv.tiles_last = stays_in_l2(a.b * a.h * a.seqlen_q * a.d * 4) && a.seqlen_k <= kMostRows;
-  p_q.tiles_last = stays_in_l2(a.b * a.h_k * a.seqlen_k * a.d * 4) && a.seqlen_q <= kMostRows;
-  auto grid_of = [&](const BwdParams &pass, int64_t seq, int64_t heads) {
-    const unsigned tiles = (unsigned)ceil_div<int64_t>(seq, 128);
-    return pass.tiles_last ? dim3((unsigned)heads, (unsigned)a.b, tiles) : dim3(tiles, (unsigned)heads, (unsigned)a.b);
-  };
-  const dim3 grid_kv = grid_of(p_kv, a.seqlen_k, a.h_k), grid_q = grid_of(p_q, a.seqlen_q, a.h);
-  auto both_passes = [&](auto bf, auto narrow) {
-    constexpr bool kBF = decltype(bf)::value, kNarrow = decltype(narrow)::value;
-    if (int rc = launch_bwd<kBF, true, kNarrow>(k_map, v_map, q64_map, do64_map, dk_map, dv_map, p_kv, grid_kv, stream))
-      return rc;
-    return launch_bwd<kBF, false, kNarrow>(q_map, do_map, k64_map, v64_map, dq_map, dq_map, p_q, grid_q, stream);
-  };
-  using std::true_type, std::false_type;
+  const BwdPass kv{(uint32_t)ceil_div<int64_t>(a.seqlen_k, 128), (uint32_t)a.h_k, (uint32_t)a.b,
+                   stays_in_l2(a.b * a.h * a.seqlen_q * a.d * 4)};
+  const BwdPass qp{(uint32_t)ceil_div<int64_t>(a.seqlen_q, kBM), (uint32_t)a.h, (uint32_t)a.b,
+                   stays_in_l2(a.b * a.h_k * a.seqlen_k * a.d * 4)};
   if (is_narrow(a.d))
-    return bf16 ? both_passes(true_type{}, true_type{}) : both_passes(false_type{}, true_type{});
-  return bf16 ? both_passes(true_type{}, false_type{}) : both_passes(false_type{}, false_type{});
+    return bf16 ? launch_bwd<true, true>(bm, p, kv, qp, stream) : launch_bwd<false, true>(bm, p, kv, qp, stream);
+  return bf16 ? launch_bwd<true, false>(bm, p, kv, qp, stream) : launch_bwd<false, false>(bm, p, kv, qp, stream);
 }

@@ -74,3 +74,42 @@ def test_short_sequences_then_dependents_of_the_decode_step(b, h, hk, d, cap, gr
         assert np.array_equal(_host(got[3]).reshape(want_k.shape), want_k[::-1])
 
     _passes(fill, chain, check, graph)
+
+
+# the backward's passes share the row sums, which another kernel leaves, and the caller's buffers of the pass before
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("b,sq,sk,h,hk,d,window", [(2, 300, 420, 8, 4, 128, (-1, -1)), (1, 1100, 1100, 16, 16, 64, (200, 0)),
+                                                   (3, 2048, 2048, 24, 8, 128, (-1, -1))])
+def test_backward_passes_in_the_same_buffers(b, sq, sk, h, hk, d, window, graph):
+    from byteir_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(sq)
+    shapes = [(b, sq, h, d), (b, sk, hk, d), (b, sk, hk, d), (b, sq, h, d)]
+    src = [[torch.randn(s, generator=gen, device="cuda").to(torch.bfloat16) for s in shapes] for _ in range(4)]
+    bufs = [torch.empty_like(t) for t in src[0]]
+    q, k, v, do = bufs
+    o, lse, dsum = torch.empty_like(q), torch.empty((b, h, sq), device="cuda"), torch.empty((b, h, (sq + 127) // 128 * 128), device="cuda")
+    grads = [torch.empty_like(t) for t in (q, k, v)]
+
+    def step(q, k, v, do, **kw):
+        fwd, bwd = ({n: kw[n] for n in names if n in kw} for names in (("out", "lse"), ("dq", "dk", "dv", "d_softmax_sum")))
+        out, l2 = ops.flash_attn_fwd(q, k, v, d ** -0.5, True, window, **fwd)
+        return (out, l2) + tuple(ops.flash_attn_bwd(do, q, k, v, out, l2, d ** -0.5, True, window, **bwd))
+
+    want = []
+    for one in src:
+        want.append(step(*one))
+        torch.cuda.synchronize()
+
+    def fill(i):
+        for dst, s in zip(bufs, src[i]):
+            dst.copy_(s)
+
+    def chain():
+        got = step(q, k, v, do, out=o, lse=lse, dq=grads[0], dk=grads[1], dv=grads[2], d_softmax_sum=dsum)
+        return got[:2] + tuple(ops.transpose(t, [0, 2, 1, 3]) for t in got[2:])
+
+    def check(i, got):
+        for g, w in zip(got, want[i][:2] + tuple(t.transpose(1, 2) for t in want[i][2:])):
+            assert torch.equal(g, w.contiguous())
+
+    _passes(fill, chain, check, graph)
