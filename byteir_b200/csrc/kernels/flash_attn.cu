@@ -1336,7 +1336,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 template <bool kBF16, bool kNarrow>
-int launch_bwd(const BwdMaps &m, const BwdParams &p, const BwdPass &kv, const BwdPass &q, cudaStream_t stream) {
+int launch_bwd(const BwdMaps &m, const BwdParams &p, const BwdPass &kv, const BwdPass &q, bool dq_over_input, cudaStream_t stream) {
   const int64_t kv_blocks = (int64_t)kv.tiles * kv.heads * kv.batch, q_blocks = (int64_t)q.tiles * q.heads * q.batch;
   if (kv_blocks + q_blocks > 0x7fffffffLL)
     return B200_ERR_UNSUPPORTED;
@@ -1345,8 +1345,14 @@ int launch_bwd(const BwdMaps &m, const BwdParams &p, const BwdPass &kv, const Bw
   if (int rc = check_cuda(cudaFuncSetAttribute(flash_bwd_kernel<kBF16, kNarrow>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)smem)))
     return rc;
-  return launch_pdl(flash_bwd_kernel<kBF16, kNarrow>, dim3((unsigned)(kv_blocks + q_blocks)), dim3(kThreads), smem, stream, m, p, kv,
-                    q, (uint32_t)kv_blocks);
+  auto go = [&](int64_t first, int64_t second) {
+    return launch_pdl(flash_bwd_kernel<kBF16, kNarrow>, dim3((unsigned)(first + second)), dim3(kThreads), smem, stream, m, p, kv, q,
+                      (uint32_t)first);
+  };
+  if (!dq_over_input)
+    return go(kv_blocks, q_blocks);
+  const int rc = go(kv_blocks, 0); // the dK/dV pass reads all of Q and dO, a dQ block only the tile that it writes
+  return rc ? rc : go(0, q_blocks);
 }
 
 } // namespace
@@ -1513,7 +1519,18 @@ extern "C" int b200_flash_attn_bwd(int dtype, const void *dout, const void *q, c
                    stays_in_l2(a.b * a.h * a.seqlen_q * a.d * 4)};
   const BwdPass qp{(uint32_t)ceil_div<int64_t>(a.seqlen_q, kBM), (uint32_t)a.h, (uint32_t)a.b,
                    stays_in_l2(a.b * a.h_k * a.seqlen_k * a.d * 4)};
+  // dQ in the place of Q or dO: one pass after the other
+  auto bytes = [&](int64_t heads, int64_t seq, int64_t hs, int64_t rs, int64_t bs) {
+    return (uintptr_t)((heads - 1) * hs + (seq - 1) * rs + (a.b - 1) * bs + a.d) * 2;
+  };
+  const uintptr_t q_bytes = bytes(a.h, a.seqlen_q, a.q_head_stride, a.q_row_stride, a.q_batch_stride);
+  const uintptr_t do_bytes = bytes(a.h, a.seqlen_q, a.o_head_stride, a.o_row_stride, a.o_batch_stride);
+  auto meets_dq = [&](const void *x, uintptr_t n) {
+    const uintptr_t d0 = reinterpret_cast<uintptr_t>(dq), x0 = reinterpret_cast<uintptr_t>(x);
+    return d0 < x0 + n && x0 < d0 + q_bytes;
+  };
+  const bool over = meets_dq(q, q_bytes) || meets_dq(dout, do_bytes);
   if (is_narrow(a.d))
-    return bf16 ? launch_bwd<true, true>(bm, p, kv, qp, stream) : launch_bwd<false, true>(bm, p, kv, qp, stream);
-  return bf16 ? launch_bwd<true, false>(bm, p, kv, qp, stream) : launch_bwd<false, false>(bm, p, kv, qp, stream);
+    return bf16 ? launch_bwd<true, true>(bm, p, kv, qp, over, stream) : launch_bwd<false, true>(bm, p, kv, qp, over, stream);
+  return bf16 ? launch_bwd<true, false>(bm, p, kv, qp, over, stream) : launch_bwd<false, false>(bm, p, kv, qp, over, stream);
 }

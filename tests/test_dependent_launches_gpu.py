@@ -113,3 +113,18 @@ def test_backward_passes_in_the_same_buffers(b, sq, sk, h, hk, d, window, graph)
             assert torch.equal(g, w.contiguous())
 
     _passes(fill, chain, check, graph)
+
+
+# dQ in the place of Q or dO: the dK/dV pass has read them before it is written
+@pytest.mark.parametrize("over", ["q", "dout"])
+def test_dq_in_the_place_of_an_input(over):
+    from byteir_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v, do = (torch.randn((2, 1500, 20, 128), generator=gen, device="cuda").to(torch.bfloat16) for _ in range(4))
+    out, lse = ops.flash_attn_fwd(q, k, v, 128 ** -0.5, True)
+    want = ops.flash_attn_bwd(do, q, k, v, out, lse, 128 ** -0.5, True)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        q2, do2 = q.clone(), do.clone()
+        got = ops.flash_attn_bwd(do2, q2, k, v, out, lse, 128 ** -0.5, True, dq=q2 if over == "q" else do2)
+        assert all(torch.equal(g, w) for g, w in zip(got, want))
