@@ -648,8 +648,10 @@ extern "C" int b200_permute(int elt_bytes, const void *in, void *out, int rank, 
     return b200_transpose_batched(elt_bytes, in, out, 1, ms[1], ms[0], stream);
   if (g == 3 && order[0] == 0 && order[1] == 2 && order[2] == 1) // (0, 2, 1)
     return b200_transpose_batched(elt_bytes, in, out, ms[0], ms[2], ms[1], stream);
-  // general case: strides of the merged input dims
-  std::vector<int64_t> in_sizes(g), in_strides(g);
+  // general case
+  if (elt_bytes != 1 && elt_bytes != 2 && elt_bytes != 4 && elt_bytes != 8)
+    return B200_ERR_UNSUPPORTED;
+  std::vector<int64_t> in_sizes(g), in_strides(g); // of the merged input dims
   for (size_t k = 0; k < g; ++k)
     in_sizes[order[k]] = ms[k];
   int64_t st = 1;
