@@ -87,8 +87,16 @@ void need_cuda(const Tensor &t) {
 Tensor new_empty(at::IntArrayRef shape, at::ScalarType type, const Tensor &like) {
   return at::detail::empty_cuda(shape, type, like.device(), std::nullopt);
 }
+// torch.empty_like, by the short way where the strides are the plain ones.  is_contiguous() does not say so: it passes over
+// dimensions of size 1, whose strides empty_like keeps (the batch of one of x[:, :s]).
 Tensor new_like(const Tensor &t) {
-  return t.is_contiguous() ? new_empty(t.sizes(), t.scalar_type(), t) : at::empty_like(t);
+  int64_t plain = 1;
+  for (int64_t i = t.dim() - 1; i >= 0; --i) {
+    if (t.stride(i) != plain)
+      return at::empty_like(t);
+    plain *= t.size(i);
+  }
+  return new_empty(t.sizes(), t.scalar_type(), t);
 }
 
 // the caller's workspace, or one of `need` bytes from torch's caching allocator (stream-ordered: it may be handed out
@@ -284,7 +292,7 @@ PyObject *index_put_add(PyObject *const *a, Py_ssize_t) {
   const Tensor *given = optional(a[4], "out"), *ws_given = optional(a[5], "workspace"), *status = optional(a[6], "status");
   Tensor made;
   if (!given)
-    made = new_empty(x.sizes(), x.scalar_type(), x);
+    made = new_like(x);
   Workspace ws(ws_given, ws_given ? 0 : b200_index_put_workspace_bytes(dt, rows, n, feature), x);
   const void *in = x.data_ptr(), *upd = update.data_ptr();
   const int64_t *idx = static_cast<const int64_t *>(index.data_ptr());
