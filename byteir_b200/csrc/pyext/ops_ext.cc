@@ -446,9 +446,17 @@ PyObject *flash_attn_bwd(PyObject *const *a, Py_ssize_t) {
   for (int i = 0; i < 4; ++i)
     given[i] = optional(a[9 + i], names[i]);
   const Tensor *like[3] = {&q, &k, &v};
-  for (int i = 0; i < 3; ++i)
+  for (int i = 0; i < 3; ++i) {
+    // The kernel writes by the strides of q, k and v.  empty_like keeps them only where the tensor is dense, which one
+    // part of a packed [B, S, 3, H, D] tensor, for instance, is not.
     if (!given[i])
-      made[i] = new_like(*like[i]);
+      made[i] = like[i]->is_non_overlapping_and_dense() ? new_like(*like[i])
+                                                        : at::empty_strided(like[i]->sizes(), like[i]->strides(), like[i]->options());
+    else if (given[i]->sizes() == like[i]->sizes())
+      for (int64_t d = 0; d < 4; ++d)
+        if (given[i]->size(d) > 1 && given[i]->stride(d) != like[i]->stride(d))
+          raise(PyExc_ValueError, "dq, dk, dv must share the strides of q, k, v");
+  }
   const b200_flash_attn_params p = attn_params(q, k, v, out, a[6], a[7], a[8]);
   if (!given[3])
     made[3] = new_empty({p.b, p.h, p.seqlen_q_rounded}, at::kFloat, q);

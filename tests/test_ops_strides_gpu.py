@@ -29,3 +29,24 @@ def test_scatter_add_output_has_the_strides_of_the_table():
     out = ops.index_put_add(x, torch.arange(50, device="cuda"), torch.ones((50, 32), device="cuda"), dim=1)
     assert out.stride() == torch.empty_like(x).stride()
     assert torch.equal(out, x + 1)
+
+
+# q, k and v as parts of one packed tensor: the gradients have their strides, and none is written past its end
+def test_gradients_of_parts_of_a_packed_tensor():
+    from byteir_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    packed = torch.randn((2, 300, 3, 4, 64), generator=gen, device="cuda").to(torch.bfloat16)
+    do = torch.randn((2, 300, 4, 64), generator=gen, device="cuda").to(torch.bfloat16)
+    q, k, v = packed.unbind(2)
+    out, lse = ops.flash_attn_fwd(q, k, v, 0.125, True)
+    grads = ops.flash_attn_bwd(do, q, k, v, out, lse, 0.125, True)
+    plain = [t.contiguous() for t in (q, k, v)]
+    out2, lse2 = ops.flash_attn_fwd(*plain, 0.125, True)
+    for g, t, w in zip(grads, (q, k, v), ops.flash_attn_bwd(do, *plain, out2, lse2, 0.125, True)):
+        assert g.stride() == t.stride() and torch.equal(g, w)
+        assert g.untyped_storage().nbytes() >= 2 * (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride())))
+    dpacked = torch.full_like(packed, 7.0)
+    got = ops.flash_attn_bwd(do, q, k, v, out, lse, 0.125, True, dq=dpacked[:, :, 0], dk=dpacked[:, :, 1], dv=dpacked[:, :, 2])
+    assert all(torch.equal(a, b) for a, b in zip(got, grads))
+    with pytest.raises(ValueError):
+        ops.flash_attn_bwd(do, q, k, v, out, lse, 0.125, True, dq=torch.empty_like(plain[0]))
