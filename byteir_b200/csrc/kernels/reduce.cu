@@ -884,8 +884,9 @@ void split_cols(ColsPlan &p, int64_t A, int64_t B) {
   p.splits = (int)ceil_div<int64_t>(supers, p.supers_per_split);
 }
 
-// Returns false where the scalar kernel is the better one.
-bool cols_plan(int esize, int64_t A, int64_t B, int64_t C, ColsPlan &p) {
+// Returns false where the scalar kernel is the better one.  `most_scratch`: bytes that the partial sums may take; a plan
+// that needs more has fewer splits, down to the eight of a cluster, which needs none.
+bool cols_plan(int esize, int64_t A, int64_t B, int64_t C, size_t most_scratch, ColsPlan &p) {
   const int N = 16 / esize;
   int64_t P = 1; // rows until the alignment repeats
   while (P * C % N != 0)
@@ -937,11 +938,20 @@ bool cols_plan(int esize, int64_t A, int64_t B, int64_t C, ColsPlan &p) {
   // thread (two latencies, less than the second launch).
   if (p.fold_rows && p.splits > 8 && std::max<int64_t>(1, B / p.P) <= 8LL * p.row_lanes * 16)
     p.splits = 8, p.supers_per_split = ceil_div<int64_t>(std::max<int64_t>(1, B / p.P), 8);
-  p.cluster = p.splits > 1 && p.splits <= 8 && (p.fold_rows || p.P == 1);
+  const bool folds = p.fold_rows || p.P == 1; // a block's sums are one per column
+  const int64_t fit = std::min<int64_t>(1 << 30, most_scratch / ((size_t)A * (folds ? 1 : p.P) * C * sizeof(float)));
+  if (p.splits > (folds ? std::max<int64_t>(8, fit) : fit)) {
+    if (!folds && fit < 1)
+      return false;
+    const int64_t supers = std::max<int64_t>(1, B / p.P);
+    p.supers_per_split = ceil_div<int64_t>(supers, folds && fit <= 8 ? 8 : fit);
+    p.splits = (int)ceil_div<int64_t>(supers, p.supers_per_split);
+  }
+  p.cluster = p.splits > 1 && p.splits <= 8 && folds;
   return true;
 }
 
-Plan make_plan(int esize, int64_t A, int64_t B, int64_t C) {
+Plan make_plan(int esize, int64_t A, int64_t B, int64_t C, size_t most_scratch = SIZE_MAX) {
   Plan p{};
   const int N = 16 / esize;
   if (C == 1) {
@@ -967,7 +977,7 @@ Plan make_plan(int esize, int64_t A, int64_t B, int64_t C) {
     p.ws_bytes = p.declared_bytes = (p.segs > 1 && !p.cluster) ? (size_t)A * p.segs * sizeof(float) : 0;
   } else {
     p.rows = false;
-    p.scalar = !cols_plan(esize, A, B, C, p.cols);
+    p.scalar = !cols_plan(esize, A, B, C, most_scratch, p.cols);
     if (!p.scalar && (p.cols.splits > 1 || !(p.cols.fold_rows || p.cols.P == 1))) {
       p.declared_bytes = (size_t)p.cols.splits * A * (p.cols.fold_rows ? 1 : p.cols.P) * C * sizeof(float);
       p.ws_bytes = p.cols.cluster ? 0 : p.declared_bytes;
@@ -978,9 +988,9 @@ Plan make_plan(int esize, int64_t A, int64_t B, int64_t C) {
 
 template <typename T, int OP, typename OutT>
 int launch(const T *in, OutT *out, int64_t A, int64_t B, int64_t C, void *ws,
-           size_t ws_bytes, cudaStream_t stream) {
+           size_t ws_bytes, size_t most_scratch, cudaStream_t stream) {
   constexpr int N = 16 / sizeof(T);
-  const Plan p = make_plan(sizeof(T), A, B, C);
+  const Plan p = make_plan(sizeof(T), A, B, C, most_scratch);
   if (p.ws_bytes > 0 && (ws == nullptr || ws_bytes < p.ws_bytes))
     return B200_ERR_WORKSPACE;
   float *partial = static_cast<float *>(ws);
@@ -1101,16 +1111,52 @@ int launch(const T *in, OutT *out, int64_t A, int64_t B, int64_t C, void *ws,
 
 template <typename T>
 int dispatch_op(int op, const void *in, void *out, int64_t A, int64_t B, int64_t C, void *ws,
-                size_t ws_bytes, cudaStream_t stream) {
+                size_t ws_bytes, size_t most_scratch, cudaStream_t stream) {
   if (op == kSum)
-    return launch<T, kSum, T>((const T *)in, (T *)out, A, B, C, ws, ws_bytes, stream);
+    return launch<T, kSum, T>((const T *)in, (T *)out, A, B, C, ws, ws_bytes, most_scratch, stream);
   if (op == kMax)
-    return launch<T, kMax, T>((const T *)in, (T *)out, A, B, C, ws, ws_bytes, stream);
+    return launch<T, kMax, T>((const T *)in, (T *)out, A, B, C, ws, ws_bytes, most_scratch, stream);
   return B200_ERR_INVALID_ARG;
 }
 
 int esize_of(int dtype) {
   return dtype == B200_F32 ? 4 : (dtype == B200_F16 || dtype == B200_BF16) ? 2 : 0;
+}
+
+int reduce_within(int op, int dtype, const void *in, void *out, int64_t A, int64_t B, int64_t C, void *workspace,
+                  size_t workspace_bytes, size_t most_scratch, cudaStream_t stream) {
+  const int es = esize_of(dtype);
+  if (!es || A < 0 || B < 0 || C < 0 || (op != kSum && op != kMax))
+    return B200_ERR_INVALID_ARG;
+  if (A == 0 && B == 0) { // nothing to reduce: a copy, as reduce_impl.h:70-73
+    if (C == 0)
+      return B200_OK;
+    if (!in || !out)
+      return B200_ERR_INVALID_ARG;
+    return check_cuda(cudaMemcpyAsync(out, in, (size_t)C * es, cudaMemcpyDeviceToDevice, stream));
+  }
+  if (A == 0 || C == 0)
+    return B200_OK; // empty output
+  if (B == 0 || !in || !out)
+    return B200_ERR_INVALID_ARG;
+  switch (dtype) {
+  case B200_F32:
+    return dispatch_op<float>(op, in, out, A, B, C, workspace, workspace_bytes, most_scratch, stream);
+  case B200_F16:
+    return dispatch_op<__half>(op, in, out, A, B, C, workspace, workspace_bytes, most_scratch, stream);
+  default:
+    return dispatch_op<__nv_bfloat16>(op, in, out, A, B, C, workspace, workspace_bytes, most_scratch, stream);
+  }
+}
+
+// The partial sums of a column reduction that splits B over one wave of blocks, each 32 vectors of a row (32 elements, if
+// a row is no whole number of vectors) wide: what b200_reduce_no_alloc measures shapes by.
+size_t plain_split_bytes(int esize, int64_t A, int64_t B, int64_t C) {
+  const int64_t units = C % (16 / esize) == 0 ? C / (16 / esize) : C;
+  const int64_t width = std::min<int64_t>(kColsThreadsPerRow, pow2_ceil(units)), blocks = A * ceil_div<int64_t>(units, width);
+  int64_t splits = std::min<int64_t>(ceil_div<int64_t>(4 * kNumSMs, blocks), std::max<int64_t>(1, B / (kBlock / width * 4)));
+  splits = ceil_div<int64_t>(B, ceil_div<int64_t>(B, splits));
+  return splits > 1 ? (size_t)splits * A * C * sizeof(float) : 0;
 }
 
 } // namespace
@@ -1153,28 +1199,7 @@ extern "C" size_t b200_reduce_scratch_bytes(int op, int dtype, int64_t A, int64_
 extern "C" int b200_reduce(int op, int dtype, const void *in, void *out, int64_t A, int64_t B,
                            int64_t C, void *workspace, size_t workspace_bytes,
                            cudaStream_t stream) {
-  const int es = esize_of(dtype);
-  if (!es || A < 0 || B < 0 || C < 0 || (op != kSum && op != kMax))
-    return B200_ERR_INVALID_ARG;
-  if (A == 0 && B == 0) { // nothing to reduce: a copy, as reduce_impl.h:70-73
-    if (C == 0)
-      return B200_OK;
-    if (!in || !out)
-      return B200_ERR_INVALID_ARG;
-    return check_cuda(cudaMemcpyAsync(out, in, (size_t)C * es, cudaMemcpyDeviceToDevice, stream));
-  }
-  if (A == 0 || C == 0)
-    return B200_OK; // empty output
-  if (B == 0 || !in || !out)
-    return B200_ERR_INVALID_ARG;
-  switch (dtype) {
-  case B200_F32:
-    return dispatch_op<float>(op, in, out, A, B, C, workspace, workspace_bytes, stream);
-  case B200_F16:
-    return dispatch_op<__half>(op, in, out, A, B, C, workspace, workspace_bytes, stream);
-  default:
-    return dispatch_op<__nv_bfloat16>(op, in, out, A, B, C, workspace, workspace_bytes, stream);
-  }
+  return reduce_within(op, dtype, in, out, A, B, C, workspace, workspace_bytes, SIZE_MAX, stream);
 }
 
 extern "C" int b200_reduce_sum_to_f32(int dtype, const void *in, float *out, int64_t A, int64_t B,
@@ -1185,12 +1210,12 @@ extern "C" int b200_reduce_sum_to_f32(int dtype, const void *in, float *out, int
     return B200_ERR_INVALID_ARG;
   switch (dtype) {
   case B200_F32:
-    return launch<float, kSum, float>((const float *)in, out, A, B, C, workspace, workspace_bytes, stream);
+    return launch<float, kSum, float>((const float *)in, out, A, B, C, workspace, workspace_bytes, SIZE_MAX, stream);
   case B200_F16:
-    return launch<__half, kSum, float>((const __half *)in, out, A, B, C, workspace, workspace_bytes, stream);
+    return launch<__half, kSum, float>((const __half *)in, out, A, B, C, workspace, workspace_bytes, SIZE_MAX, stream);
   default:
     return launch<__nv_bfloat16, kSum, float>((const __nv_bfloat16 *)in, out, A, B, C, workspace,
-                                              workspace_bytes, stream);
+                                              workspace_bytes, SIZE_MAX, stream);
   }
 }
 
@@ -1248,14 +1273,20 @@ int static_scratch_for_current_device(void **ptr) {
 
 extern "C" size_t b200_reduce_no_alloc_max_bytes(void) { return kStaticScratchBytes; }
 
+// Takes what fits by either measure: the plan's own scratch or that of a plain split, and makes a plan that fits.
 extern "C" int b200_reduce_no_alloc(int op, int dtype, const void *in, void *out, int64_t A, int64_t B,
                                     int64_t C, cudaStream_t stream) {
-  const size_t need = b200_reduce_workspace_bytes(op, dtype, A, B, C);
-  if (need > kStaticScratchBytes)
-    return B200_ERR_WORKSPACE; // this shape needs more scratch than the fixed block holds
+  const int es = esize_of(dtype);
+  size_t need = 0;
+  if (es && A > 0 && B > 0 && C > 0) {
+    if (b200_reduce_workspace_bytes(op, dtype, A, B, C) > kStaticScratchBytes &&
+        (C == 1 || plain_split_bytes(es, A, B, C) > kStaticScratchBytes))
+      return B200_ERR_WORKSPACE;
+    need = make_plan(es, A, B, C, kStaticScratchBytes).ws_bytes;
+  }
   void *scratch = nullptr;
   if (need > 0)
     if (int rc = static_scratch_for_current_device(&scratch))
       return rc;
-  return b200_reduce(op, dtype, in, out, A, B, C, scratch, need ? kStaticScratchBytes : 0, stream);
+  return reduce_within(op, dtype, in, out, A, B, C, scratch, need ? kStaticScratchBytes : 0, kStaticScratchBytes, stream);
 }

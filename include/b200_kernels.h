@@ -119,8 +119,9 @@ int b200_sharded_sum_finish(int dtype, const float *partial, void *const *peer_i
  * fixed block of b200_reduce_no_alloc_max_bytes() (1 MiB) of device memory that is
  * part of the library image; every GPU that loads the library holds that block
  * until the process exits.  The call allocates and frees nothing.
- *  - A shape whose b200_reduce_workspace_bytes() exceeds the block is refused with
- *    B200_ERR_WORKSPACE; nothing is launched.
+ *  - A shape is served where b200_reduce_workspace_bytes() fits the block, and where
+ *    the partial sums of B split over one wave of blocks do (with fewer splits then).
+ *    Others are refused with B200_ERR_WORKSPACE; nothing is launched.
  *  - The first call made with a given device current looks up the block's device
  *    address (a host-side query, no device work).  Make that first call before any
  *    stream capture begins.
