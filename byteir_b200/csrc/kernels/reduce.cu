@@ -12,17 +12,18 @@
 //                        one thread-block cluster through distributed shared
 //                        memory (single launch, no workspace); more segments go
 //                        through f32 partials in the workspace and a second pass.
-//   C  > 1  ("columns"): a warp reads one (or several short) contiguous rows of a
-//                        column slab per step, 8 warps stride over the B rows,
-//                        and B is split over enough blocks to fill 148 SMs
-//                        (split-K); the f32 partials of the splits are combined in
-//                        split order by a second pass, so the result does not
-//                        depend on scheduling.  (Folding in the first launch - the
-//                        last block of a slab to finish, found by a ticket, folds
-//                        it - was measured slower: 14.4 against 13.6 us on f16
-//                        [32768, 1024], because the fence, the ticket and the fold
-//                        are one more latency chain after the last load, while
-//                        the second pass is already resident and waiting.)
+//   C  > 1  ("columns"): few rows, or columns enough for a thread each, are walked
+//                        over by one thread per vector; otherwise threads sum
+//                        super-rows (as many rows as make whole vectors) and B is
+//                        split over enough blocks to fill 148 SMs.  Up to eight
+//                        splits fold through distributed shared memory; more leave
+//                        f32 partials, which a second pass folds in split order, so
+//                        that the result does not depend on scheduling.  (Folding in
+//                        the first launch - the last block of a slab to finish, found
+//                        by a ticket, folds it - was measured slower: 14.4 against
+//                        13.6 us on f16 [32768, 1024], because the fence, the ticket
+//                        and the fold are one more latency chain after the last load,
+//                        while the second pass is already resident and waiting.)
 //
 // Max semantics (reduction_helper.h:159-180 folded in ascending index order):
 // NaN wins; otherwise the largest value; between +0 and -0, which compare equal,
@@ -488,30 +489,36 @@ template <typename T, int OP> struct Vec16 {
 };
 
 // A maximum that is exactly zero takes the sign of the last zero of its column (the hardware max
-// ranks -0 below +0): a backward scan of rows [lo, hi) that ends at that zero, sixteen loads in flight.
-template <typename T> __device__ float last_zero(const T *col, int64_t lo, int64_t hi, int64_t C) {
-  for (int64_t r = hi - 1; r >= lo; r -= 16) {
-    float v[16];
+// ranks -0 below +0): a backward scan of rows [lo, hi) that ends at that zero, LOADS of them in flight.
+template <int LOADS, typename T> __device__ __forceinline__ float scan_for_zero(const T *col, int64_t lo, int64_t hi, int64_t C) {
+#pragma unroll 1
+  for (int64_t r = hi - 1; r >= lo; r -= LOADS) {
+    float v[LOADS];
 #pragma unroll
-    for (int u = 0; u < 16; ++u)
+    for (int u = 0; u < LOADS; ++u)
       v[u] = r - u >= lo ? Elt<T>::to_f32(col[(r - u) * C]) : 1.f;
 #pragma unroll
-    for (int u = 0; u < 16; ++u)
+    for (int u = 0; u < LOADS; ++u)
       if (v[u] == 0.f)
         return v[u];
   }
   return 0.f;
 }
+// Out of line: it is rare, and its registers cost the two kernels that use it blocks per SM.  (The kernels of super-rows, at
+// their limit of 64 registers, are 10 % slower with a call in them.)
+template <typename T> __device__ __noinline__ float last_zero(const T *col, int64_t hi, int64_t C) {
+  return scan_for_zero<16>(col, 0, hi, C);
+}
 // The same where the rows are split over blocks: the last zero lies in the rows of the last split whose maximum is zero, and
 // only those are scanned (all rows, one by one, of f16 [32768, 1024] with one zero in front took 7.1 ms a call, now 52 us).  `run`: the
 // matrix, `split`: that split, `split_elems`: the elements of one, the last one's end `super` or fewer behind it.
 template <typename T>
-__device__ float last_zero_of_split(const T *run, int64_t c, int split, int splits, int64_t split_elems, int64_t super, int64_t B,
+__device__ __forceinline__ float last_zero_of_split(const T *run, int64_t c, int split, int splits, int64_t split_elems, int64_t super, int64_t B,
                                     int64_t C) {
   const int64_t total = B * C, head = min(total, (int64_t)elements_to_boundary(run));
   const int64_t begin = split == 0 ? 0 : max((int64_t)0, min(head + split * split_elems, total - super));
   const int64_t end = split == splits - 1 ? total : min(total, head + (split + 1) * split_elems);
-  return last_zero(run + c, begin / C, min(B, (end + C - 1) / C), C); // a row too many on either side changes nothing
+  return scan_for_zero<8>(run + c, begin / C, min(B, (end + C - 1) / C), C); // a row too many on either side changes nothing
 }
 
 template <typename T, int OP, int VPT, bool CLUSTER, typename OutT>
@@ -676,8 +683,89 @@ __global__ void __launch_bounds__(512, 2)
   }
 }
 
-// Element by element, for the few shapes where super-rows do not pay (see cols_plan): four columns and
-// four rows in flight per thread.
+// One thread per 16-byte vector of the output's columns (VEC), or per column, for all B rows: no fold, no barrier, eight
+// loads in flight.  For few rows, and for so many columns that the threads fill the chip (see cols_plan).  The eight rows of a
+// batch are folded in pairs, so that a sum's chain has B / 8 additions, as many as where eight warps share the rows.
+template <typename T, int OP, bool VEC, typename OutT>
+__global__ void __launch_bounds__(kBlock)
+    reduce_cols_direct_kernel(const T *__restrict__ in, OutT *__restrict__ out, int64_t units, int64_t B, int64_t C, int64_t per_row,
+                              FastDiv by_row) {
+  constexpr int N = VEC ? 16 / sizeof(T) : 1;
+  pdl_launch_dependents();
+  const int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x;
+  const bool ok = i < units;
+  const int64_t a = units < (1LL << 31) ? (int64_t)by_row.quot((uint32_t)i) : i / per_row;
+  const T *p = in + (ok ? a * B * C + (i - a * per_row) * N : 0);
+  if (ok)
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (u < B)
+        prefetch_l2(p + u * C);
+  pdl_wait();
+  if (!ok)
+    return;
+  float acc[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    acc[j] = op_init<OP>();
+  auto value = [](const auto &v, int j) -> float { // element j of a loaded unit
+    if constexpr (!VEC) {
+      return Elt<T>::to_f32(v);
+    } else {
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      if constexpr (sizeof(T) == 4)
+        return __uint_as_float(w[j]);
+      else if constexpr (std::is_same<T, __half>::value)
+        return __half2float(__ushort_as_half((unsigned short)(w[j >> 1] >> (j & 1) * 16)));
+      else
+        return __uint_as_float(j & 1 ? w[j >> 1] & 0xffff0000u : w[j >> 1] << 16);
+    }
+  };
+  for (int64_t r = 0; r < B; r += 8, p += 8 * C) {
+    typename std::conditional<VEC, uint4, T>::type x[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (r + u < B) {
+        if constexpr (VEC)
+          x[u] = ld_nc_v4(p + u * C);
+        else
+          x[u] = p[u * C];
+      }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      float s[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        s[u] = r + u < B ? value(x[u], j) : op_init<OP>();
+#pragma unroll
+      for (int half = 4; half > 0; half /= 2)
+#pragma unroll
+        for (int u = 0; u < half; ++u)
+          s[u] = op_combine<OP>(s[u], s[u + half]);
+      acc[j] = op_combine<OP>(acc[j], s[0]);
+    }
+  }
+  if (OP == kMax)
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (acc[j] == 0.f)
+        acc[j] = last_zero(in + a * B * C + (i - a * per_row) * N + j, B, C);
+  OutT *o = out + i * N;
+  if constexpr (VEC) {
+    __align__(16) OutT v[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      v[j] = Elt<OutT>::from_f32(acc[j]);
+#pragma unroll
+    for (int k = 0; k < (int)(N * sizeof(OutT) / 16); ++k)
+      reinterpret_cast<uint4 *>(o)[k] = reinterpret_cast<const uint4 *>(v)[k];
+  } else {
+    store_out(o, acc[0]);
+  }
+}
+
+// Eight warps share the rows, element by element, four columns and four rows in flight per thread: where super-rows do not
+// pay and there are too few columns for a thread each (see cols_plan).
 constexpr int kScalarCols = 4;
 template <typename T, int OP, typename OutT>
 __global__ void __launch_bounds__(kBlock)
@@ -718,7 +806,7 @@ __global__ void __launch_bounds__(kBlock)
     for (int w = 1; w < 8; ++w)
       r = op_combine<OP>(r, sums[w][i]);
     if (OP == kMax && r == 0.f)
-      r = last_zero(run + c0 + i, 0, B, C);
+      r = last_zero(run + c0 + i, B, C);
     store_out(out + a * C + c0 + i, r);
   }
 }
@@ -858,6 +946,7 @@ int g_rows_blocks_per_sm = 4;
 int g_reserved_blocks = 0;
 
 // ---- launch plan: a pure function of the shape -----------------------------
+enum ColsPath { kSuper, kScalar, kDirect };
 struct Plan {
   bool rows;
   // rows
@@ -865,7 +954,7 @@ struct Plan {
   int64_t seg_len;
   bool cluster;
   // columns
-  bool scalar;
+  ColsPath path;
   ColsPlan cols;
   size_t ws_bytes;      // what the launch uses
   size_t declared_bytes; // what b200_reduce_workspace_bytes says
@@ -884,10 +973,21 @@ void split_cols(ColsPlan &p, int64_t A, int64_t B) {
   p.splits = (int)ceil_div<int64_t>(supers, p.supers_per_split);
 }
 
-// Returns false where the scalar kernel is the better one.  `most_scratch`: bytes that the partial sums may take; a plan
-// that needs more has fewer splits, down to the eight of a cluster, which needs none.
-bool cols_plan(int esize, int64_t A, int64_t B, int64_t C, size_t most_scratch, ColsPlan &p) {
+// `most_scratch`: bytes that the partial sums may take; a plan that needs more has fewer splits, down to the eight of a
+// cluster, which needs none.
+ColsPath cols_plan(int esize, int64_t A, int64_t B, int64_t C, size_t most_scratch, ColsPlan &p) {
   const int N = 16 / esize;
+  // A thread per unit (a vector, or an element where rows are no whole vectors) walks over B rows, eight per round trip; eight
+  // warps share them with the scalar kernel; super-rows start with more work per block and split further.  Measured on 446
+  // shapes, us by a thread per unit / eight warps / super-rows: f32 [628, 2, 14604] 24 / 125 / 271, bf16 max [302, 4, 1280]
+  // 3.0 / 8.3 / 10.0, f32 max [387, 73, 2325] 52 / 66 / 419; f16 max [5, 28, 88] 5.2 / 2.2 / 3.0, bf16 [358, 30691]
+  // 17.2 / 14.4 / 19.2; f16 [34721, 1848] 3872 / 1921 / 22.
+  const bool whole = C % N == 0;
+  const int64_t units = whole ? A * C / N : A * C;
+  if (whole ? B <= 8 || units >= 8LL * kNumSMs * B : B <= 16 || (B <= 32 && units >= 2048) || units >= 200 * B)
+    return kDirect;
+  if (C >= 32 && B <= (whole ? 32 : 64)) // with fewer columns most lanes of a warp would idle
+    return kScalar;
   int64_t P = 1; // rows until the alignment repeats
   while (P * C % N != 0)
     P *= 2;
@@ -907,8 +1007,8 @@ bool cols_plan(int esize, int64_t A, int64_t B, int64_t C, size_t most_scratch, 
   } else {
     // slabs of 32 vectors; every column's P partial sums go through the workspace, which is worth it while they are
     // few against the B rows
-    if (P > 1 && B < 16 * P)
-      return false;
+    if (P > 1 && (B < 16 * P || (B <= 512 && 2 * units >= kNumSMs * B)))
+      return kScalar;
     p.P = P;
     p.nvec = nvec;
     p.vpt = 1;
@@ -942,13 +1042,13 @@ bool cols_plan(int esize, int64_t A, int64_t B, int64_t C, size_t most_scratch, 
   const int64_t fit = std::min<int64_t>(1 << 30, most_scratch / ((size_t)A * (folds ? 1 : p.P) * C * sizeof(float)));
   if (p.splits > (folds ? std::max<int64_t>(8, fit) : fit)) {
     if (!folds && fit < 1)
-      return false;
+      return kScalar;
     const int64_t supers = std::max<int64_t>(1, B / p.P);
     p.supers_per_split = ceil_div<int64_t>(supers, folds && fit <= 8 ? 8 : fit);
     p.splits = (int)ceil_div<int64_t>(supers, p.supers_per_split);
   }
   p.cluster = p.splits > 1 && p.splits <= 8 && folds;
-  return true;
+  return kSuper;
 }
 
 Plan make_plan(int esize, int64_t A, int64_t B, int64_t C, size_t most_scratch = SIZE_MAX) {
@@ -977,8 +1077,8 @@ Plan make_plan(int esize, int64_t A, int64_t B, int64_t C, size_t most_scratch =
     p.ws_bytes = p.declared_bytes = (p.segs > 1 && !p.cluster) ? (size_t)A * p.segs * sizeof(float) : 0;
   } else {
     p.rows = false;
-    p.scalar = !cols_plan(esize, A, B, C, most_scratch, p.cols);
-    if (!p.scalar && (p.cols.splits > 1 || !(p.cols.fold_rows || p.cols.P == 1))) {
+    p.path = cols_plan(esize, A, B, C, most_scratch, p.cols);
+    if (p.path == kSuper && (p.cols.splits > 1 || !(p.cols.fold_rows || p.cols.P == 1))) {
       p.declared_bytes = (size_t)p.cols.splits * A * (p.cols.fold_rows ? 1 : p.cols.P) * C * sizeof(float);
       p.ws_bytes = p.cols.cluster ? 0 : p.declared_bytes;
     }
@@ -1069,7 +1169,19 @@ int launch(const T *in, OutT *out, int64_t A, int64_t B, int64_t C, void *ws,
     }
     return B200_OK;
   }
-  if (p.scalar) {
+  if (p.path == kDirect) {
+    const bool vec = C % N == 0 && aligned16(in) && aligned16(out);
+    const int64_t per_row = vec ? C / N : C, units = A * per_row, blocks = ceil_div<int64_t>(units, kBlock);
+    if (blocks > 0x7fffffffLL)
+      return B200_ERR_UNSUPPORTED;
+    const FastDiv by_row((uint32_t)std::min<int64_t>(per_row, 0x7fffffff));
+    if (vec)
+      return launch_pdl(reduce_cols_direct_kernel<T, OP, true, OutT>, dim3((unsigned)blocks), dim3(kBlock), 0, stream, in, out, units, B,
+                        C, per_row, by_row);
+    return launch_pdl(reduce_cols_direct_kernel<T, OP, false, OutT>, dim3((unsigned)blocks), dim3(kBlock), 0, stream, in, out, units, B, C,
+                      per_row, by_row);
+  }
+  if (p.path == kScalar) {
     const int64_t slabs = ceil_div<int64_t>(C, 32 * kScalarCols);
     if (A * slabs > 0x7fffffffLL)
       return B200_ERR_UNSUPPORTED;
