@@ -664,10 +664,15 @@ __global__ void __launch_bounds__(256)
 
 // Short lists: the whole sort in one block, which keeps the list in shared memory between the passes (digits of 8 bits).
 // It is bound by latency, its own passes' (about 1 us each) instead of five dependent kernels' and their launches'; the
-// sorted list is the same.  f32 [100000, 64] x 1000 in place 22.3 -> 15.0 us, f16 [1500, 33] x 300 28.5 -> 21.2.  Beside a
-// table copy up to as many entries as the block holds (f32 [500000, 64] x 8192 71 -> 51: one kernel waits behind the copy
-// instead of five), in place up to half of them: f16 [100000, 64] x 8192 27.6 us with five kernels, 30.2 with one.
+// sorted list is the same.  f32 [100000, 64] x 1000 in place 22.3 -> 15.0 us, f16 [1500, 33] x 300 28.5 -> 21.2.
 constexpr int kSmallSort = 8192; // entries: 1024 threads x 8
+// How many entries it takes, us with five kernels / with one.  In place 4096: f16 [100000, 64] x 8192 27.6 / 30.2.  Beside a table
+// copy 5120 (f16 [375000, 16] x 4500 28.7 / 25.6, x 6000 29.7 / 30.8, x 8192 30.2 / 37.1), and as many as it holds where the
+// copy is long enough, because one kernel waits behind it and not five: f32 [187500, 64] (48 MB) x 8192 41.3 / 37.2, [375000, 64]
+// 55.1 / 40.1, but [93750, 64] (24 MB) 32.2 / 36.4.
+int64_t small_sort_entries(bool in_place, int64_t table_bytes) {
+  return in_place ? 4096 : table_bytes >= 40000000 ? kSmallSort : 5120;
+}
 constexpr int kSmallRadixBits = 8, kSmallRadix = 1 << kSmallRadixBits;
 struct SmallSortShared {
   uint32_t key[kSmallSort];
@@ -1476,7 +1481,7 @@ int scatter_add(const T *in, const int64_t *idx, const T *upd, T *out, int64_t r
   const int nb = (int)p.nblocks;
   const int radix = 1 << p.digit_bits;
   int cur = 0;
-  if (n <= (in != out ? kSmallSort : kSmallSort / 2)) {
+  if (n <= small_sort_entries(in == out, rows * feature * (int64_t)sizeof(T))) {
     // the attribute belongs to the current device's context: set on every call (a host-side table write)
     if (int rc = check_cuda(cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)sizeof(SmallSortShared))))

@@ -21,3 +21,15 @@ def test_short_lists(n, rows):
         t, i, u = torch.from_numpy(table).cuda(), torch.from_numpy(ids.astype(np.int64)).cuda(), torch.from_numpy(upd).cuda()
         assert np.array_equal(ops.index_put_add(t, i, u).cpu().numpy(), want)
         assert np.array_equal(ops.index_put_add(t, i, u, out=t).cpu().numpy(), want)
+
+
+# beside a table copy one block sorts 5120 entries, and 8192 from 40 MB of table on
+@pytest.mark.parametrize("rows,feature", [(9000, 33), (156249, 64), (156250, 64)])
+@pytest.mark.parametrize("n", [5120, 5121, 8192, 8193])
+def test_lists_around_the_most_that_one_block_sorts(n, rows, feature):
+    from byteir_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(n + rows)
+    table, upd = (torch.randint(-8, 8, (k, feature), generator=gen, device="cuda").float() for k in (rows, n))
+    ids = torch.randint(0, rows, (n,), generator=gen, device="cuda")
+    ids[: n // 4] = ids[0]
+    assert torch.equal(ops.index_put_add(table, ids, upd), table.index_add(0, ids, upd))
