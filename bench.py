@@ -328,7 +328,7 @@ class ReduceC2Sum(ReduceBase):
     """f16 [64, 512, 1024] N(0,1): ReduceSum over dims {0,1} (column reduction, f32 accumulate) -> f16 [1024]"""
     key, name, dtype = "reduce_c2_sum", "reduce_f16_64x512x1024_sum01", "f16 (f32 accumulate)"
     op, shape, dims = "sum", (64, 512, 1024), (0, 1)
-    kernel = "reduce_cols_kernel + reduce_finalize_kernel"
+    kernel = "reduce_cols_kernel + reduce_cols_fold_kernel"
     launches = 2
 
     def host_inputs(self, n):
@@ -353,7 +353,7 @@ class ReduceC2(Workload):
     """f16 [64, 512, 1024] N(0,1): ReduceSum dims {0,1} -> f16 [1024] and ReduceMax dim 2 -> f16 [64, 512]; under
     N ranks the global tensor is [64 N, 512, 1024], dim 0 sharded, so the sum ends with an exchange of partials"""
     key, name, dtype = "reduce_c2", "reduce_f16_64x512x1024_sum01_max2", "f16 (f32 accumulate)"
-    kernel = "reduce_cols_kernel + reduce_finalize_kernel (ReduceSum dims {0,1})"
+    kernel = "reduce_cols_kernel + reduce_cols_fold_kernel (ReduceSum dims {0,1})"
 
     def __init__(self, rank, world, rows0=64):
         super().__init__(rank, world)

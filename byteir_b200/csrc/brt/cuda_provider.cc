@@ -20,6 +20,9 @@
 #include <cstring>
 #include <dlfcn.h>
 
+// what a launch uses, which can be less than b200_reduce_workspace_bytes; not in the header
+extern "C" size_t b200_reduce_scratch_bytes(int op, int dtype, int64_t A, int64_t B, int64_t C);
+
 namespace brt {
 namespace cuda {
 
@@ -112,7 +115,7 @@ public:
     for (size_t i = 0; i < passes_.size(); ++i) {
       const Pass &p = passes_[i];
       if (p.A && p.B && p.C)
-        kernel_ws_ = std::max(kernel_ws_, b200_reduce_workspace_bytes(OP, i == 0 ? in_dtype_ : mid, p.A, p.B, p.C));
+        kernel_ws_ = std::max(kernel_ws_, b200_reduce_scratch_bytes(OP, i == 0 ? in_dtype_ : mid, p.A, p.B, p.C));
     }
     kernel_ws_ = (kernel_ws_ + 255) & ~(size_t)255;
     mid_bytes_ = 0;

@@ -468,7 +468,7 @@ int launch_short(const void *in, void *out, int64_t batch, int64_t rows, int64_t
   while ((2ll << lw) * shorts * ES <= kShortBytes && (1ll << lw) < len && batch * ceil_div<int64_t>(len, 2ll << lw) >= 2 * kNumSMs)
     ++lw;
   const int64_t pieces = ceil_div<int64_t>(len, 1ll << lw);
-  if (batch * pieces > 0x7fffffffLL) // more pieces than a grid has blocks: the tiles are walked by a fixed grid
+  if (batch * pieces > 0x7fffffffLL) // more pieces than a grid dimension has blocks: tiles, the batch in two dimensions
     return launch_tile<ES>(in, out, batch, rows, cols, stream);
   const size_t smem = (size_t)shorts * ((1 << lw) + 16 / ES) * ES;
   const bool vec = len * ES % 16 == 0 && aligned16(from_rows ? in : out);

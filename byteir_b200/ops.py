@@ -38,31 +38,6 @@ def _need_cuda(*ts):
             raise ValueError("tensors must be contiguous (ByRE memrefs are)")
 
 
-def reduce_abc(shape, dimensions):
-    """A x B x C view of reduce_impl.h:28-59.  Dimensions of size 1 are taken out of the shape first, so
-    that reduced dimensions with only such dimensions between them count as consecutive."""
-    keep = [i for i, s in enumerate(shape) if s != 1]
-    renumber = {d: k for k, d in enumerate(keep)}
-    dims = sorted({renumber[d] for d in dimensions if shape[d] != 1})
-    if not dims:
-        n = 1
-        for s in shape:
-            n *= s
-        return 0, 0, n
-    shape = [shape[i] for i in keep]
-    for a, b in zip(dims, dims[1:]):
-        if b - a != 1:
-            raise ValueError("Only consecutive dimensions reduction is supported")
-    A = B = Cc = 1
-    for s in shape[:dims[0]]:
-        A *= s
-    for d in dims:
-        B *= shape[d]
-    for s in shape[dims[-1] + 1:]:
-        Cc *= s
-    return A, B, Cc
-
-
 def reduce_sum(x, dimensions, out=None, workspace=None):
     return _X.reduce(N.REDUCE_SUM, x, dimensions, out, workspace)
 
@@ -138,7 +113,11 @@ def flash_attn_kvcache(q, kcache, vcache, knew=None, vnew=None, seqlens_k=None, 
                        causal=True, window=(-1, -1), out=None, lse=None, workspace=None):
     """One decode step: append knew/vnew [B, S_new, H_k, D] to the caches [B, S_max, H_k, D] at row
     seqlens_k[b] (i32 [B]; None = the cache is full and nothing is appended) and attend q [B, Sq, H, D]
-    to the rows in use.  The caches are updated in place.  Returns (out, softmax_lse[B, H, Sq])."""
+    to the rows in use.  The caches are updated in place.  Returns (out, softmax_lse[B, H, Sq]).
+
+    Where blocks share the keys of the batch equally (large caches, head dims 64 and 128) the parts in which a
+    sequence is summed follow from the lengths of all sequences.  The same batch gives the same bits; the same
+    sequence beside others gives the same result to within the rounding of 16-bit probabilities."""
     return _X.flash_attn_kvcache(q, kcache, vcache, knew, vnew, seqlens_k, softmax_scale, causal, window, out, lse,
                                  workspace)
 

@@ -246,7 +246,10 @@ int b200_flash_attn_take_status(int *status);
  * seqlens_k[b] + seqlen_knew rows, the mask aligned to the end of the keys; new rows
  * that would not fit the cache are dropped.  D is a multiple of 8, at most 256.
  * workspace: scratch of b200_flash_attn_kvcache_workspace_bytes(params) bytes, or NULL
- * to take it from the stream's memory pool for the duration of the call. */
+ * to take it from the stream's memory pool for the duration of the call.
+ * A batch gives the same bits on every call.  In large caches the parts in which a
+ * sequence is summed depend on the lengths of all sequences, so beside other ones its
+ * result differs by the rounding of 16-bit probabilities. */
 typedef struct {
   int64_t q_batch_stride, k_batch_stride, v_batch_stride, knew_batch_stride, vnew_batch_stride, o_batch_stride;
   int64_t q_row_stride, k_row_stride, v_row_stride, knew_row_stride, vnew_row_stride, o_row_stride;

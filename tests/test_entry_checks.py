@@ -55,3 +55,33 @@ def test_no_alloc_results(A, B, C, dt, op):
         mag += x[:, i:i + 256].double().abs().sum(1)
     bound = {"f32": 0.0, "f16": 2.0**-11, "bf16": 2.0**-8}[dt] * want.abs() * 1.001 + 2.0**-24 * (B / 8 + 32) * mag
     assert bool(((got.double() - want).abs() <= bound).all())
+
+
+# a module's reduction takes the scratch that its launch uses: none where the splits fold through distributed shared memory
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,used", [((64, 1000, 256), False), ((1, 32768, 1024), True)])
+def test_module_takes_the_scratch_that_its_launch_uses(shape, used):
+    import torch
+    from byteir_b200 import _native as N, brt
+    from test_brt_host import reduce_mlir
+    sizes = []
+
+    def alloc(size):
+        sizes.append(size)
+        return torch.cuda.caching_allocator_alloc(max(size, 1))
+
+    declared = N.lib().b200_reduce_workspace_bytes(N.REDUCE_SUM, N.F16, *shape)
+    assert declared > 0
+    out_shape = (shape[0], shape[2])
+    s = brt.Session("cuda", alloc_func=alloc, free_func=torch.cuda.caching_allocator_delete)
+    s.load_from_memory(reduce_mlir("ReduceSumOp_f16_f16", "f16", shape, out_shape, "dense<1> : tensor<1xi64>"))
+    x, out = torch.randn(shape, device="cuda").half(), torch.empty(out_shape, device="cuda", dtype=torch.float16)
+    request = s.new_request(torch.cuda.current_stream().cuda_stream)
+    request.bind_args([(0, x.data_ptr()), (1, out.data_ptr())])
+    request.finish_io_binding()
+    request.run()
+    torch.cuda.synchronize()
+    torch.testing.assert_close(out.float(), x.float().sum(1), rtol=2e-2, atol=1e-2)
+    assert sum(sizes) == ((declared + 255) // 256 * 256 if used else 0)
+    request.close()
+    s.close()
