@@ -357,7 +357,7 @@ constexpr int kLeastShare = 4;                  // steps: below that a block's s
 // a sequence follow from all lengths, and with them the running maxima that probabilities are rounded against: beside other
 // sequences a result differs by that rounding (0.2 % in the norm for bf16; against float64 the error is that of ranges,
 // 0.00218 and 0.00220 on the first example below).
-// bf16 [16 entries of 4096..8191 keys, 32 / 8 heads, 128]: 103 -> 89 us (3920 -> 4530 GB/s); [1 of 30000]: 45 -> 39;
+// bf16 [16 entries of 4096..8191 keys, 32 / 8 heads, 128]: 103 -> 89..91 us (3920 -> 4440..4530 GB/s); [1 of 30000]: 45 -> 39;
 // f16 [16 of 1200..6000, 16 / 16, 64]: 70 -> 64.  Two blocks share an SM, so a thread may have 255 registers (it uses 216).
 struct Shares {
   int total, share; // steps of all entries and heads; per block
